@@ -261,12 +261,8 @@ def prepare(case: dict, seed: int) -> dict:
             albedos = {k: tuple(map(float, r.uniform(0.05, 0.85, 3))) for k in ("red", "green", "white", "base")}
             sc = scenes.cornell_box(case["width"], case["height"], albedos=albedos)
         else:
-            # the benchmark's terrain; the seed chooses the paths.  510 sky
-            # rows: 1 / (1 / 510) rounds below 510 in float32, so a direction
-            # straight down (latitude exactly 1) falls in the last row of the
-            # sky's importance distribution whether or not the renderer clamps
-            # the index; with 512 a renderer that does not reads past the rows
-            sc = scenes.terrain_scene(case["width"], case["height"], env_w=1020, env_h=510)
+            # the benchmark's own terrain; the seed chooses the paths
+            sc = scenes.terrain_scene(case["width"], case["height"])
         ds = state["scene"] = DeviceScene(sc, device)
         state["states"] = _pixel_states(ds.width * ds.height, seed, device)
     return state
