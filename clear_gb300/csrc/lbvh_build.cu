@@ -2239,6 +2239,12 @@ extern "C" int clr_lbvh_build_batched(clr_lbvh* h, const float* vx, const float*
 constexpr int kRayKeyBits = 8;
 constexpr int kRayPasses = 3;
 
+// Rays sorted at a time (whole tiles): the sort's look-back words carry counts
+// below 2^30 under two flag bits, and rays of one origin all count under one
+// digit.  Longer lists are sorted and searched in parts of this many.
+constexpr uint32_t kMaxSortRays = (1u << 30) - 4096u;
+static_assert(kMaxSortRays <= kValueMask && kMaxSortRays % (kSortThreads * SortCfg<uint32_t>::kItems) == 0, "");
+
 __global__ void __launch_bounds__(256) k_ray_keys(const float4* __restrict__ rays, uint32_t n,
                                                   const float* __restrict__ root_box, uint32_t* __restrict__ keys,
                                                   unsigned int* __restrict__ hist) {
@@ -2351,7 +2357,24 @@ int clr_trace_shadow_in_order(const clr_bvh* bvh, const float* rays, uint32_t nu
 
 extern "C" int clr_trace_sort_workspace_bytes(uint32_t num_rays, uint64_t* bytes) {
     if (!bytes) return clr_set_error(CLR_EINVAL, "clr_trace_sort_workspace_bytes: bytes is NULL");
-    *bytes = ray_sort_layout(num_rays, nullptr, nullptr);
+    *bytes = ray_sort_layout(std::min(num_rays, kMaxSortRays), nullptr, nullptr);
+    return CLR_OK;
+}
+
+// Sorts and searches a list part by part: search(first, n, order) takes the n
+// rays from `first` on in their order.
+template <class Search>
+static int trace_sorted(const clr_bvh* bvh, const float* rays, uint32_t num_rays, void* workspace,
+                        uint64_t workspace_bytes, void* stream, Search search) {
+    for (uint32_t first = 0; first < num_rays;) {
+        const uint32_t n = std::min(num_rays - first, kMaxSortRays);
+        const uint32_t* order = nullptr;
+        int rc = ray_order(bvh, rays ? rays + 8ull * first : nullptr, n, workspace, workspace_bytes,
+                           static_cast<cudaStream_t>(stream), &order);
+        if (rc == CLR_OK) rc = search(first, n, order);
+        if (rc != CLR_OK) return rc;
+        first += n;
+    }
     return CLR_OK;
 }
 
@@ -2359,22 +2382,23 @@ extern "C" int clr_trace_closest_sorted(const clr_bvh* bvh, const float* rays, u
                                         float* hit_t, void* workspace, uint64_t workspace_bytes, void* stream) {
     if (num_rays == 0) return clr_trace_closest_in_order(bvh, rays, 0, nullptr, hit_id, hit_t, stream);
     if (!bvh || bvh->num_tris == 0) return clr_trace_closest_in_order(bvh, rays, num_rays, nullptr, hit_id, hit_t, stream);
-    const uint32_t* order = nullptr;
-    cudaStream_t st = static_cast<cudaStream_t>(stream);
-    int rc = ray_order(bvh, rays, num_rays, workspace, workspace_bytes, st, &order);
-    if (rc != CLR_OK) return rc;
-    return clr_trace_closest_in_order(bvh, rays, num_rays, order, hit_id, hit_t, stream);
+    return trace_sorted(bvh, rays, num_rays, workspace, workspace_bytes, stream,
+                        [&](uint32_t first, uint32_t n, const uint32_t* order) {
+                            return clr_trace_closest_in_order(bvh, rays + 8ull * first, n, order,
+                                                              hit_id ? hit_id + first : nullptr,
+                                                              hit_t ? hit_t + first : nullptr, stream);
+                        });
 }
 
 extern "C" int clr_trace_shadow_sorted(const clr_bvh* bvh, const float* rays, uint32_t num_rays, uint8_t* occluded,
                                        void* workspace, uint64_t workspace_bytes, void* stream) {
     if (num_rays == 0) return clr_trace_shadow_in_order(bvh, rays, 0, nullptr, occluded, stream);
     if (!bvh || bvh->num_tris == 0) return clr_trace_shadow_in_order(bvh, rays, num_rays, nullptr, occluded, stream);
-    const uint32_t* order = nullptr;
-    cudaStream_t st = static_cast<cudaStream_t>(stream);
-    int rc = ray_order(bvh, rays, num_rays, workspace, workspace_bytes, st, &order);
-    if (rc != CLR_OK) return rc;
-    return clr_trace_shadow_in_order(bvh, rays, num_rays, order, occluded, stream);
+    return trace_sorted(bvh, rays, num_rays, workspace, workspace_bytes, stream,
+                        [&](uint32_t first, uint32_t n, const uint32_t* order) {
+                            return clr_trace_shadow_in_order(bvh, rays + 8ull * first, n, order,
+                                                             occluded ? occluded + first : nullptr, stream);
+                        });
 }
 
 extern "C" int clr_lbvh_export_reference(clr_lbvh* h, const clr_bvh* bvh, void* inodes, void* lnodes,

@@ -236,7 +236,9 @@ CLR_API int clr_trace_shadow(const clr_bvh* bvh, const float* rays, uint32_t num
  * smaller ones up to 1.1x (4 M triangles) or nothing (1 M); for rays already
  * ordered (a camera's) a cost of about a millisecond per 16 M rays.  The
  * 256-byte aligned device workspace holds clr_trace_sort_workspace_bytes(n)
- * bytes (16 per ray and the sort's tile words); its contents are scratch. */
+ * bytes (16 per ray and the sort's tile words); its contents are scratch.
+ * Lists of 2^30 rays and more are sorted and searched in parts that share the
+ * workspace, which therefore stops growing there. */
 CLR_API int clr_trace_sort_workspace_bytes(uint32_t num_rays, uint64_t* bytes);
 CLR_API int clr_trace_closest_sorted(const clr_bvh* bvh, const float* rays, uint32_t num_rays, uint32_t* hit_id,
                                      float* hit_t, void* workspace, uint64_t workspace_bytes, void* stream);
