@@ -65,14 +65,14 @@ __global__ void __launch_bounds__(128) k_trace_counted(DScene sc, const float4* 
                                                        uint32_t* __restrict__ hit_id, uint32_t* __restrict__ counts) {
     const uint32_t r = blockIdx.x * blockDim.x + threadIdx.x;
     if (r >= n) return;
-    const float4 a = rays[2u * r], b = rays[2u * r + 1];
+    const float4 a = rays[2ull * r], b = rays[2ull * r + 1];
     uint2 stack[kStackSize];
     uint32_t cnt[2] = {0u, 0u};
     Hit h;
     const bool hit = intersect_impl<false, true>(sc, mk(a.x, a.y, a.z), mk(b.x, b.y, b.z), h, stack, cnt);
     if (hit_id) hit_id[r] = hit ? h.id : kNone32;
-    counts[2u * r] = cnt[0];
-    counts[2u * r + 1] = cnt[1];
+    counts[2ull * r] = cnt[0];
+    counts[2ull * r + 1] = cnt[1];
 }
 
 }  // namespace clr

@@ -82,7 +82,7 @@ namespace clr {
 constexpr uint32_t kLeafBit = 0x80000000u;
 }  // namespace clr
 
-static inline unsigned int div_up(unsigned int a, unsigned int b) { return (a + b - 1) / b; }
+static inline unsigned int div_up(unsigned int a, unsigned int b) { return a / b + (a % b != 0u); }
 
 // Streaming multiprocessors of the current device (capi.cu), queried once per
 // device; grids that fill the GPU once are sized from it.

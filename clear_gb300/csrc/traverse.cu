@@ -49,7 +49,7 @@ struct ListIo {
         return true;
     }
     __device__ __forceinline__ Ray ray(uint32_t q) const { return load_ray(rays, q); }
-    __device__ __forceinline__ float4 dir(uint32_t q) const { return __ldg(rays + 2u * q + 1u); }
+    __device__ __forceinline__ float4 dir(uint32_t q) const { return __ldg(rays + 2ull * q + 1u); }
     __device__ __forceinline__ void done(uint32_t q, const Tree&, float t, uint32_t best) const {
         hit_id[q] = best;
         hit_t[q] = t;

@@ -16,7 +16,7 @@ struct Ray {
 };
 
 __device__ __forceinline__ Ray load_ray(const float4* rays, uint32_t r) {
-    const float4 a = __ldg(rays + 2u * r), b = __ldg(rays + 2u * r + 1u);
+    const float4 a = __ldg(rays + 2ull * r), b = __ldg(rays + 2ull * r + 1u);
     return Ray{a.x, a.y, a.z, a.w, b.x, b.y, b.z};
 }
 

@@ -75,3 +75,22 @@ def test_sorted_lists_above_2_30_rays(cuda):
     assert _lib.device_status() == 0
     del rays
     torch.cuda.empty_cache()
+
+
+@pytest.mark.gpu
+def test_lists_above_2_31_rays(cuda):
+    """Ray r's record is floats 8 r to 8 r + 7: float4 2 r, beyond 32 bits here."""
+    n = (1 << 31) + 4099
+    bvh, few, rays = _long_list(cuda, n, one_origin=False)
+    for ordered in (True, False):
+        ids, ts = lbvh.trace_closest(bvh, rays, ordered=ordered)
+        want_id, want_t = lbvh.trace_closest(bvh, few, ordered=ordered)
+        assert _repeats(ids, want_id) and _repeats(ts.view(torch.int32), want_t.view(torch.int32)), ordered
+        del ids, ts
+    assert _repeats(lbvh.trace_shadow(bvh, rays), lbvh.trace_shadow(bvh, few))
+    ids, counts = lbvh.trace_closest_counted(bvh, rays)
+    want_id, want_counts = lbvh.trace_closest_counted(bvh, few)
+    assert _repeats(ids, want_id) and _repeats(counts, want_counts)
+    assert _lib.device_status() == 0
+    del rays, ids, counts
+    torch.cuda.empty_cache()
