@@ -238,9 +238,11 @@ __device__ __forceinline__ uint32_t shade_class(const DScene& sc, uint32_t id) {
     if (id == kNone32) return 0u;
     const uint32_t mat = __ldg(reinterpret_cast<const uint32_t*>(sc.faces + 56u * (size_t)id) + 13) & 0xFFFFu;
     const uint8_t* m = sc.materials + mat;
-    const uint32_t num = m[0], first = m[8];  // MaterialInfo is 8 bytes, the first element's id follows
-    return num == 0 ? 1u : num == 1 ? 2u + min(first, 1u) + (first == kBxNewWard ? 1u : 0u)
-                                    : 5u + (first == kBxDiffuse ? 0u : first == kBxAshS ? 1u : 2u);
+    const uint32_t num = m[0];
+    if (num == 0) return 1u;  // the blob may end with the 8 bytes of its MaterialInfo
+    const uint32_t first = m[8];  // the first element's id
+    return num == 1 ? 2u + min(first, 1u) + (first == kBxNewWard ? 1u : 0u)
+                    : 5u + (first == kBxDiffuse ? 0u : first == kBxAshS ? 1u : 2u);
 }
 
 // The entry of a queue of n, binned by bin_chunk, that thread i of the shading
