@@ -410,6 +410,20 @@ __device__ __forceinline__ uint32_t node_boxes(const Node& nd, const SlabRay& k,
     return acc;
 }
 
+// node_boxes with exact entries, by box_test_fast alone.
+__device__ __forceinline__ uint32_t node_boxes_woo(const Node& nd, const Ray& r, const SlabRay& k, float& e0, float& e1) {
+    float a[6], b[6], ix, iy, iz;
+    unpack2(k.iv_xy, ix, iy);
+    unpack2(k.iv_yz, iy, iz);
+#pragma unroll
+    for (int j = 0; j < 3; ++j) {
+        unpack2(nd.b0[j], a[2 * j], a[2 * j + 1]);
+        unpack2(nd.b1[j], b[2 * j], b[2 * j + 1]);
+    }
+    return (box_test_fast(a[0], a[1], a[2], a[3], a[4], a[5], r, ix, iy, iz, e0) ? 1u : 0u) |
+           (box_test_fast(b[0], b[1], b[2], b[3], b[4], b[5], r, ix, iy, iz, e1) ? 2u : 0u);
+}
+
 // The root's box (root_box of clr_bvh), as node_boxes.
 template <bool kBounded = false, class GetRay>
 __device__ __forceinline__ bool root_box_hit(const float* root_box, const SlabRay& k, GetRay ray, bool exact, float& e,
