@@ -75,11 +75,12 @@ __device__ __forceinline__ bool light_on_ray(const DScene& sc, uint32_t face, co
     const float mxx = fmaxf(p0.x, fmaxf(p1.x, p2.x)), mxy = fmaxf(p0.y, fmaxf(p1.y, p2.y)),
                 mxz = fmaxf(p0.z, fmaxf(p1.z, p2.z));
     // an upper bound needs no classification: box_test's entry is the largest
-    // quotient of an outside axis, within 6u of the largest lo
+    // quotient of an outside axis, within 6u of the largest lo (NaN where the
+    // origin lies on a plane of an axis the ray is parallel to)
     auto get_ray = [&]() { return ray; };
     float e;
     slab_test(pack2(mnx, mny), pack2(mnz, mxx), pack2(mxy, mxz), slab, get_ray, false, e);
-    G = slab.mr < INFINITY ? e * kEntryUp : INFINITY;
+    G = slab.mr < INFINITY && e == e ? e * kEntryUp : INFINITY;
     return true;
 }
 
