@@ -1,11 +1,12 @@
 """Autotuner of the batched form.
 
 Picks, for one batch on one GPU, the path-slot pool size (the queue
-capacity), the block sizes of the tracing and shading kernels and the radix
-width of the segmented LBVH sort, by timing candidates on the batch itself
-(CUDA events, a 1-sample frame per render candidate) in coordinate-descent
-order: pool size, then trace block, then shade block; radix width for the
-build.  Results are cached in a JSON file keyed by the GPU and the batch's
+capacity), the block sizes of the per-ray tracing kernels and of the shading
+kernel and the radix width of the segmented LBVH sort, by timing candidates on
+the batch itself (CUDA events, a 1-sample frame per render candidate) in
+coordinate-descent order: pool size, then trace block (only where some scene
+has cutouts: the other batches are searched over block pools of a fixed block
+size), then shade block; radix width for the build.  Results are cached in a JSON file keyed by the GPU and the batch's
 shape (scenes, pixels, triangles, depth), so a later run of the same
 workload skips the search.
 """
@@ -90,6 +91,8 @@ def tune(br, max_depth: int = 5, use_cache: bool = True, graph: bool = True) -> 
     cfg = {"trace_block": 128, "shade_block": 128, "pool_slots": 0}
     for field, values in (("pool_slots", POOL_CANDIDATES), ("trace_block", TRACE_BLOCKS),
                           ("shade_block", SHADE_BLOCKS)):
+        if field == "trace_block" and getattr(br, "pool_searches", False):
+            continue
         best_v, best_ms = cfg[field], None
         for v in values:
             c = dict(cfg, **{field: v})
