@@ -635,18 +635,29 @@ static unsigned int bt_grid(uint32_t work, uint32_t block) {
     return std::max(1u, std::min(div_up(work, block), (unsigned int)clr_sm_count() * (2048u / block)));
 }
 
+// Grids of the pool searches, if the batch takes them: asked for once a render
+// (the runtime's occupancy query), not once an iteration.
+struct BtGrids {
+    bool pool;
+    unsigned int extend, shadow;
+};
+
+static BtGrids bt_grids(const clr_batch* b, bool ordered) {
+    if (!ordered || b->alpha) return BtGrids{false, 0u, 0u};
+    const unsigned int work = div_up(b->slots, 4);
+    return BtGrids{true, resident_grid(k_bt_extend_pool, kSearchThreads, 0, work),
+                   resident_grid(k_bt_shadow_pool, kSearchThreads, 0, work)};
+}
+
 // One iteration's kernels (parity cur).  In a graph the shadow rays run on a
 // second branch, beside the next iteration's extension, and are joined before
 // the next shade kernel (the caller joins the last).  With the pool searches:
 // 64 scenes of random triangles, 2 samples 105 -> 71.5 ms.
-static void bt_iteration(const clr_batch* b, const BtArgs& A, int cur, bool ordered, cudaStream_t st,
+static void bt_iteration(const clr_batch* b, const BtArgs& A, const BtGrids& g, int cur, bool ordered, cudaStream_t st,
                          const GraphFork* fork, bool join) {
     const uint32_t tb = b->cfg.trace_block, sb = b->cfg.shade_block;
     const unsigned int gt = bt_grid(b->slots, tb), gs = bt_grid(b->slots, sb);
-    const bool pool = ordered && !b->alpha;
-    if (pool)
-        k_bt_extend_pool<<<resident_grid(k_bt_extend_pool, kSearchThreads, 0, div_up(b->slots, 4)), kSearchThreads, 0,
-                           st>>>(A, b->S, cur);
+    if (g.pool) k_bt_extend_pool<<<g.extend, kSearchThreads, 0, st>>>(A, b->S, cur);
     else if (ordered) k_bt_extend<true><<<gt, tb, 0, st>>>(A, b->S, cur);
     else k_bt_extend<false><<<gt, tb, 0, st>>>(A, b->S, cur);
     k_bt_bin<<<std::min(2u * (unsigned int)clr_sm_count(), div_up(b->slots, (uint32_t)kBinChunk)), kBinChunk, 0, st>>>(
@@ -654,9 +665,7 @@ static void bt_iteration(const clr_batch* b, const BtArgs& A, int cur, bool orde
     if (fork && join) fork->join(st);
     k_bt_shade<<<gs, sb, 0, st>>>(A, b->S, cur);
     cudaStream_t side = fork ? fork->begin(st) : st;
-    if (pool)
-        k_bt_shadow_pool<<<resident_grid(k_bt_shadow_pool, kSearchThreads, 0, div_up(b->slots, 4)), kSearchThreads, 0,
-                           side>>>(A, b->S, cur);
+    if (g.pool) k_bt_shadow_pool<<<g.shadow, kSearchThreads, 0, side>>>(A, b->S, cur);
     else if (ordered) k_bt_shadow<true><<<gt, tb, 0, side>>>(A, b->S, cur);
     else k_bt_shadow<false><<<gt, tb, 0, side>>>(A, b->S, cur);
 }
@@ -689,6 +698,7 @@ static int bt_capture(clr_batch* b, const BtArgs& A, bool ordered, unsigned int 
     if (!b->capture) CLR_CUDA_TRY(cudaStreamCreateWithFlags(&b->capture, cudaStreamNonBlocking));
     if (!b->fork.make()) return clr_set_error(CLR_ECUDA, "clr_batch_render: capture stream or events");
     cudaStream_t st = b->capture;
+    const BtGrids grids = bt_grids(b, ordered);
     cudaGraph_t g = nullptr;
     CLR_CUDA_TRY(cudaGraphCreate(&g, 0));
     cudaGraphConditionalHandle h;
@@ -720,7 +730,7 @@ static int bt_capture(clr_batch* b, const BtArgs& A, bool ordered, unsigned int 
         cudaGraph_t body = cp.conditional.phGraph_out[0];
         e = cudaStreamBeginCaptureToGraph(st, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal);
         if (e == cudaSuccess) {
-            for (int k = 0; k < kBtBodyIters; ++k) bt_iteration(b, A, k & 1, ordered, st, &b->fork, k > 0);
+            for (int k = 0; k < kBtBodyIters; ++k) bt_iteration(b, A, grids, k & 1, ordered, st, &b->fork, k > 0);
             b->fork.join(st);
             k_bt_continue<<<1, 1, 0, st>>>(b->S, h, max_iters);
             cudaGraph_t out = nullptr;
@@ -771,9 +781,10 @@ extern "C" int clr_batch_render(clr_batch* b, uint32_t* rand_states, float* pixe
     }
     k_bt_init<<<bt_grid(b->slots, b->cfg.trace_block), b->cfg.trace_block, 0, st>>>(A, b->S);
     CLR_LAUNCH_CHECK("k_bt_init");
+    const BtGrids grids = bt_grids(b, ordered);
     for (uint64_t it = 0; it < cap; ++it) {
         const int cur = (int)(it & 1);
-        bt_iteration(b, A, cur, ordered, st, nullptr, false);
+        bt_iteration(b, A, grids, cur, ordered, st, nullptr, false);
         CLR_LAUNCH_CHECK("batched iteration");
         if ((it & 7) == 7) {
             unsigned int left = 0;
