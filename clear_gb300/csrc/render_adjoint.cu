@@ -320,8 +320,8 @@ __device__ __forceinline__ void ad_clear_counts(const AdState& S, int cur) {
     }
 }
 
-// Closest hit of every queued path of both passes.
-template <bool kOrdered>
+// Closest hit of every queued path of both passes, ray by ray in the reference's
+// order, in which scenes with cutouts are always searched.
 __global__ void __launch_bounds__(kAdThreads, 8) k_ad_extend(DScene sc, AdState S, int cur, int cached) {
     const uint32_t n0 = S.count[2 * cur], n = n0 + S.count[2 * cur + 1];
     ad_clear_counts(S, cur);
@@ -339,7 +339,7 @@ __global__ void __launch_bounds__(kAdThreads, 8) k_ad_extend(DScene sc, AdState 
         }
         const float4 o = S.org[p], d = S.dir[p];
         Hit h;
-        if (intersect<kOrdered>(sc, mk(o.x, o.y, o.z), mk(d.x, d.y, d.z), h, stack))
+        if (intersect<false>(sc, mk(o.x, o.y, o.z), mk(d.x, d.y, d.z), h, stack))
             S.hit[p] = make_float4(__uint_as_float(h.id), h.t, h.b1, h.b2);
         else
             S.hit[p] = make_float4(__uint_as_float(kNone32), INFINITY, 0.f, 0.f);
@@ -1082,8 +1082,7 @@ static void ad_block(const AdArgs& a, cudaStream_t st, const GraphFork* fork) {
     for (int k = 0; k < kAdBlockIters; ++k) {
         const int cur = k & 1;
         if (a.pool) k_ad_extend_pool<<<a.grid_extend, kSearchThreads, 0, st>>>(a.sc, a.S, cur, a.cached);
-        else if (a.ordered) k_ad_extend<true><<<a.grid, kAdThreads, 0, st>>>(a.sc, a.S, cur, a.cached);
-        else k_ad_extend<false><<<a.grid, kAdThreads, 0, st>>>(a.sc, a.S, cur, a.cached);
+        else k_ad_extend<<<a.grid, kAdThreads, 0, st>>>(a.sc, a.S, cur, a.cached);
         k_ad_bin<<<a.grid_bin, kBinChunk, 0, st>>>(a.sc, a.S, cur);
         if (fork && k > 0) fork->join(st);  // the previous shadow work
         cudaStream_t side = fork ? fork->begin(st) : st;

@@ -149,7 +149,8 @@ __global__ void __launch_bounds__(kSearchThreads, kWfExtendBlocks) k_wf_extend_p
     search_nearer(io, n, sp, sh, over);
 }
 
-template <bool kOrdered>
+// Ray by ray in the reference's order, in which scenes with cutouts are always
+// searched.
 __global__ void __launch_bounds__(kWfThreads, 8) k_wf_extend(DScene sc, WfState S, int cur) {
     const uint32_t n = S.count[4 * cur + kActive];
     wf_clear_counts(S, cur);
@@ -158,7 +159,7 @@ __global__ void __launch_bounds__(kWfThreads, 8) k_wf_extend(DScene sc, WfState 
         const uint32_t p = S.q[cur][i];
         const float4 o = S.org[p], d = S.dir[p];
         Hit h;
-        if (intersect<kOrdered>(sc, mk(o.x, o.y, o.z), mk(d.x, d.y, d.z), h, stack))
+        if (intersect<false>(sc, mk(o.x, o.y, o.z), mk(d.x, d.y, d.z), h, stack))
             S.hit[p] = make_float4(__uint_as_float(h.id), h.t, h.b1, h.b2);
         else
             S.hit[p] = make_float4(__uint_as_float(kNone32), INFINITY, 0.f, 0.f);
@@ -461,8 +462,7 @@ static void wf_block(const WfArgs& a, cudaStream_t st, const GraphFork* fork) {
     for (int k = 0; k < kWfBlockIters; ++k) {
         const int cur = k & 1;
         if (a.pool) k_wf_extend_pool<<<a.grid_trace, kSearchThreads, 0, st>>>(a.sc, a.S, cur);
-        else if (a.ordered) k_wf_extend<true><<<a.grid_trace, kWfThreads, 0, st>>>(a.sc, a.S, cur);
-        else k_wf_extend<false><<<a.grid_trace, kWfThreads, 0, st>>>(a.sc, a.S, cur);
+        else k_wf_extend<<<a.grid_trace, kWfThreads, 0, st>>>(a.sc, a.S, cur);
         k_wf_partition<<<a.grid_bin, kBinChunk, 0, st>>>(a.sc, a.S, a.S.q[cur], cur, a.pool);
         if (fork && k > 0) fork->join(st);  // the previous shadow rays
         cudaStream_t side = fork ? fork->begin(st) : st;
@@ -531,10 +531,10 @@ extern "C" int clr_render_wavefront_rows(const clr_scene* scene, uint32_t width,
         grid_trace = resident_grid(k_wf_extend_pool, kSearchThreads, 0, div_up(npix, 4));
         grid_shadow = resident_grid(k_wf_shadow_pool, kSearchThreads, 0, div_up(npix, 4));
     } else {
-        grid_trace = grid_shadow = ordered ? std::min(resident_grid(k_wf_extend<true>, kWfThreads, 0, work),
-                                                      resident_grid(k_wf_shadow<true>, kWfThreads, 0, work))
-                                           : std::min(resident_grid(k_wf_extend<false>, kWfThreads, 0, work),
-                                                      resident_grid(k_wf_shadow<false>, kWfThreads, 0, work));
+        grid_trace = grid_shadow =
+            std::min(resident_grid(k_wf_extend, kWfThreads, 0, work),
+                     ordered ? resident_grid(k_wf_shadow<true>, kWfThreads, 0, work)
+                             : resident_grid(k_wf_shadow<false>, kWfThreads, 0, work));
     }
     const WfArgs a{sc, S, width, row0, spp, max_depth, rand_states, px, ordered, pool, grid, grid_trace, grid_shadow,
                    std::min(2u * (unsigned int)clr_sm_count(), div_up(npix, kBinChunk))};
