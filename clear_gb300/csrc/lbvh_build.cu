@@ -567,9 +567,9 @@ __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)_
 // -> 51 / 53 us (the host's share of a call is about 48).
 //
 // Block c owns positions [c * kTile, (c + 1) * kTile); each pass ranks its keys
-// as k_onesweep does (warp multisplit, stable), reads every block's digit
-// totals, and stores each key and value straight into the shared memory of the
-// block that owns its new position.
+// stably (a ballot a digit bit finds the lanes of a warp with the same digit),
+// reads every block's digit totals, and stores each key and value straight into
+// the shared memory of the block that owns its new position.
 constexpr int kClusterThreads = 1024, kClusterWarps = kClusterThreads / 32;
 constexpr int kClusterMaxBlocks = 8;  // the portable cluster size
 constexpr int kClusterMaxItems = 2;   // keys per thread
@@ -1873,7 +1873,6 @@ static int run_build(clr_lbvh* h, const float* vx, const float* vy, const float*
         else
             rc = launch_sort_cluster<KeyT, 2>(h, vx, vy, vz, tri, n, bits, npasses, dst, st);
         if (rc != CLR_OK) return rc;
-        timer.done("box_morton_sort");
     } else {
         constexpr bool k64 = sizeof(KeyT) == 8;
         const bool small = n <= (k64 ? kSmallSortKeys64 : kSmallSortKeys32);
@@ -2046,8 +2045,15 @@ extern "C" int clr_lbvh_host_copy_wait(clr_lbvh* h) {
     return CLR_OK;
 }
 
-// Batches with at least this many triangles a scene are sorted scene by scene
-// (a scene then fills a quarter of its last tile on average at the least).
+// Batches with a mean of at least this many triangles a scene are sorted scene by
+// scene.  They have at most n / 4,096 + n / 1,024 tiles (n / 2,048 + n / 1,024 with
+// 64-bit keys), so the tiles are a fifth (a third) full on average at the least,
+// however uneven the scenes are.  Composite keys against scene by scene, 10 bits:
+// 1,000 scenes of 1,024 triangles 265 / 225 us, one of 1 Mi and 1,000 of one
+// triangle 285 / 268, one of 4 Mi and 4,000 of two 880 / 780; but 8 of 5,000 88 / 95.
+// The line could lie lower: 1,000 scenes of 600 triangles 218 / 184, even at about
+// 130 to 470 keys a tile (one of 256 Ki and 2,000 of three 161 / 161; two of 256 Ki
+// and 1,000 of three 193 / 202).
 constexpr uint32_t kSegSortMinTris = 1024;
 
 // Words of histograms and look-back that a sort scene by scene of up to `cap`
