@@ -164,21 +164,19 @@ __device__ __forceinline__ bool tri_hit(const float4* __restrict__ tris, uint32_
 // With u = 2^-24 and 1 / d from rcp.approx (2u), an estimate is within 4u of
 // the real quotient (relative; its sign is exact), box_test's quotients within
 // 2u, and its point o + maxt d within u (2 |maxt d| + |o|) of the real one.
-// Let M = max_k |o_k / d_k| over the nonzero d_k, mr = 2^-23 M + 1e-30 = 2u M (the
-// constant covers products that underflow), tp = max(tn, 0), below = (1 - 2^-19)
-// tp - mr and above = (1 + 2^-19) tp + mr (margins of 32u tp), and second = the
-// larger of 0 and the second largest lo.  Then
-//   tf < below      tn <= 0: a slab lies behind the origin, which moves away
-//                   from it; tn > 0: the point at maxt lies outside axis tf's
-//                   slab by more than its rounding: box_test rejects;
-//   tn < -mr and tf > above
-//                   the origin is inside all slabs: box_test accepts with entry
-//                   -inf;
-//   tf > above and second < below
-//                   maxt is the quotient of tn's axis alone (the others lie
-//                   below it by more than the errors, and it is within 6u of
-//                   tn) and the point at maxt lies inside the other two slabs
-//                   by more than its rounding: accepted;
+// Let M = max_k |o_k / d_k| over the nonzero d_k, mr = 2^-23 M + 1e-30, m = 2^-19 |tn|
+// + mr = 32u |tn| + 2u M (the constant covers products that underflow), tn+ =
+// max(tn, 0), and second = the larger of 0 and the second largest lo.  Then
+//   tf - tn+ <= -m  either tf <= -m: the origin lies beyond a slab the ray moves
+//                   away from; or tn - tf >= m: the point at maxt lies outside
+//                   axis tf's slab by more than its rounding: box_test rejects;
+//   tf - tn+ > m and |tn| - second > m
+//                   either tn < -m and tf > m: the origin is inside all slabs,
+//                   box_test accepts with entry -inf; or maxt is the quotient
+//                   of tn's axis alone (the others lie below it by more than
+//                   the errors, and it is within 6u of tn) and the point at
+//                   maxt lies inside the other two slabs by more than its
+//                   rounding: accepted;
 // anything else is unsure: grazing and corner hits, flat boxes entered through
 // their flat axis, origins on a plane.  (tn's own axis passes box_test by t ==
 // maxt, so for tn > 0 the tf of the other two axes will do: slab_flat_hit, on
@@ -188,17 +186,19 @@ __device__ __forceinline__ bool tri_hit(const float4* __restrict__ tris, uint32_
 // A zero component needs no margin: its 1 / d is infinite, so the axis gives lo
 // = -inf, hi = inf where the origin lies between the planes (box_test's point
 // keeps that coordinate, and the axis takes no part), both infinite with one
-// sign where it does not (tf = -inf, or below = inf: a miss, as in box_test), and
-// NaN where the origin is on a plane.  With the axis in M instead, and so no box
-// sure, rays parallel to an axis were up to 2.5 times slower than by box_test
-// alone; before the classification / so / now, 4 Mi vertical rays on 2 Mi
-// triangles of a terrain mesh: closest hit 5.9 / 8.5 / 4.3 ms, shadow 4.4 / 7.7 /
-// 4.1, an orthographic camera's 4.4 / 7.6 / 4.1.  Components that are tiny but not
-// zero keep their large M: within about 1e-5 of an axis most boxes are unsure.
+// sign where it does not (tf - tn+ = -inf <= -m, also where m is infinite with tn: a
+// miss, as in box_test), and NaN where the origin is on a plane.  With that axis
+// in M instead no box was sure, and rays parallel to an axis were up to 2.5 times
+// slower than by box_test alone: before the classification / so / now, 4 Mi
+// vertical rays on 2 Mi triangles of a terrain mesh, closest hit 5.8 / 8.5 / 4.3
+// ms, shadow 4.4 / 7.7 / 4.1; an orthographic camera's 4.3 / 7.6 / 3.2 and 3.0 / 6.8 /
+// 3.2.
+// Components that are tiny but not zero keep their large M: within about 1e-5 of
+// an axis most boxes are unsure (the vertical rays tilted by 1e-7: 6.0 / 8.4 / 8.4).
 //
 // NaN anywhere (min / max propagate it) and rays with a nonzero d outside [2^-40,
-// 2^40] in magnitude (mr infinite) fail every test.  (An estimate past the float
-// range counts as larger than any finite one.)
+// 2^40] in magnitude or an infinite M (mr is NaN) fail both tests.  An estimate
+// past the float range counts as larger than any finite one.
 typedef unsigned long long f32x2;  // two packed floats, the lower one first
 
 __device__ __forceinline__ f32x2 pack2(float a, float b) {
@@ -265,10 +265,9 @@ __device__ __forceinline__ SlabRay make_slab_ray(const Ray& r) {
     k.iv_yz = pack2(iy, iz);
     const float ax = r.dx == 0.0f ? 0.0f : fabsf(ix), ay = r.dy == 0.0f ? 0.0f : fabsf(iy),
                 az = r.dz == 0.0f ? 0.0f : fabsf(iz);  // zero components take no part
-    const float hi = max_nan(ax, ay, az);
+    const float lo = min_nan(fabsf(ix), fabsf(iy), fabsf(iz)), hi = max_nan(ax, ay, az);
     const float M = max_nan(fabsf(r.ox) * ax, fabsf(r.oy) * ay, fabsf(r.oz) * az);
-    const float dm = max_nan(fabsf(r.dx), fabsf(r.dy), fabsf(r.dz));
-    k.mr = (hi <= 0x1p40f && dm <= 0x1p40f) ? M * 0x1p-23f + 1e-30f : INFINITY;
+    k.mr = (hi <= 0x1p40f && lo >= 0x1p-40f && M < INFINITY) ? M * 0x1p-23f + 1e-30f : __int_as_float(0x7FFFFFFF);
     return k;
 }
 
@@ -298,11 +297,11 @@ __device__ __forceinline__ int slab_test(f32x2 p0, f32x2 p1, f32x2 p2, const Sla
     const float lxy = max_nan(lx, ly);
     const float tn = max_nan(lxy, lz);
     const float second = max_nan(min_nan(lx, ly), min_nan(lxy, lz), 0.0f);
-    const float tp = max_nan(tn, 0.0f);
-    const float below = __fmaf_rn(tp, 1.0f - 0x1p-19f, -k.mr), above = __fmaf_rn(tp, 1.0f + 0x1p-19f, k.mr);
-    const bool miss = tf < below;
-    const bool inside = tn < -k.mr;
-    const bool hit = tf > above && (inside || second < below);
+    const float m = __fmaf_rn(fabsf(tn), 0x1p-19f, k.mr);
+    const float d = tf - max_nan(tn, 0.0f), g = fabsf(tn) - second;
+    const bool miss = d <= -m;
+    const bool hit = d > m && g > m;
+    const bool inside = tn < 0.0f;
     entry = inside ? -INFINITY : tn;
     if (exact && hit && !inside) {
         // the quotient of tn's axis (alone: the other lo lie below tn - m)
