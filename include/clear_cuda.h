@@ -161,10 +161,14 @@ CLR_API int clr_lbvh_build_noalloc(const float* vx, const float* vy, const float
  * triangles [scene_offsets[s], scene_offsets[s+1]) of the concatenated inputs
  * (`tri` holds indices into the concatenated vertex arrays, or is NULL for a
  * soup); scene_offsets is a HOST array of num_scenes + 1 entries starting at
- * 0, every scene non-empty.  One scene-box pass, one Morton pass (keys carry
- * the scene id above the 3 x bits_per_dim Morton bits), one radix sort of
- * radix_bits-bit digits (6, 7 or 8; 0 = 8) and one tree pass build every
- * scene.  Scene s's BVH is
+ * 0, every scene non-empty.  One scene-box pass, one Morton pass, one radix sort
+ * of radix_bits-bit digits (6, 7 or 8; 0 = 8; scene by scene, or for batches with
+ * a mean below 1,024 triangles a scene on keys that carry the scene id above the
+ * 3 x bits_per_dim Morton bits, which together must fit 64 bits and eight digits
+ * in either case)
+ * and one tree pass build every scene.  The builder's scratch grows with the
+ * triangles and the scenes, not with the split: a call of no more of either than
+ * before allocates nothing.  Scene s's BVH is
  *   {n_s, bits_per_dim, nodes + CLR_NODE_BYTES * off_s,
  *    tris + CLR_TRI_BYTES * off_s, root_boxes + 8 * s}
  * (triangle ids scene-local) and is bit-identical to clr_lbvh_build of that
